@@ -81,18 +81,21 @@ struct dcf_ctx {
 
 // the context whose API call is running on this thread (for prof_begin/prof_end)
 static thread_local dcf_ctx *t_active = nullptr;
-static thread_local bool t_launched = false;  // follows_launch()
+static thread_local bool t_launched = false;                // follows_launch()
+static thread_local cudaError_t t_failed = cudaSuccess;     // first failed launch of the running call
 struct ActiveScope {
     dcf_ctx *prev;
     explicit ActiveScope(dcf_ctx *c) : prev(t_active)
     {
         t_active = c;
         t_launched = false;
+        t_failed = cudaSuccess;
     }
     ~ActiveScope()
     {
         t_active = prev;
         t_launched = false;
+        t_failed = cudaSuccess;
     }
 };
 
@@ -117,8 +120,13 @@ static void prof_record(int id, bool begin, cudaStream_t s)
 namespace dcf {
 void prof_begin(int id, cudaStream_t s) { prof_record(id, true, s); }
 void prof_end(int id, cudaStream_t s) { prof_record(id, false, s); }
-void note_launch()
+bool may_launch() { return t_failed == cudaSuccess; }
+void note_launch(cudaError_t e)
 {
+    if (e != cudaSuccess) {
+        if (t_active) t_failed = e;
+        return;
+    }
     if (t_active) t_active->launches++;
     t_launched = t_active != nullptr;
 }
@@ -230,6 +238,7 @@ static cudaError_t dmalloc_async(dcf_ctx *c, T **p, size_t bytes, cudaStream_t s
 static dcf_status check_launch(dcf_ctx *ctx, int)
 {
     cudaError_t e = cudaGetLastError();
+    if (t_failed != cudaSuccess) e = t_failed;
     if (e != cudaSuccess) return set_err(ctx, DCF_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
     return DCF_OK;
 }
@@ -924,7 +933,7 @@ dcf_status dcf_tree_parent(dcf_ctx *ctx, dcf_tree *t, int64_t *parent, int on_de
         if (st != DCF_OK) return st;
         dst = (long long *)s;
     }
-    k_widen<<<grid_for(t->g.N, 256, ctx->sm_count), 256, 0, ctx->stream>>>(t->g.N, t->parent, dst); note_launch();
+    launch_plain(k_widen, grid_for(t->g.N, 256, ctx->sm_count), 256, 0, ctx->stream, t->g.N, t->parent, dst);
     dcf_status st = check_launch(ctx, 1);
     if (st != DCF_OK) return st;
     if (!on_device) CU(cudaMemcpyAsync(parent, dst, N * 8, cudaMemcpyDeviceToHost, ctx->stream));
@@ -2225,8 +2234,8 @@ dcf_status dcf_batch_parent(dcf_ctx *ctx, dcf_batch *b, int64_t *parent, int on_
         if ((st = scratch(ctx, 10, N * 8, &sbuf)) != DCF_OK) return st;
         dst = (long long *)sbuf;
     }
-    k_batch_local_parent<<<grid_for(b->N, 256, ctx->sm_count), 256, 0, ctx->stream>>>(b->N, b->parent, b->d_offs,
-                                                                                      b->count, dst); note_launch();
+    launch_plain(k_batch_local_parent, grid_for(b->N, 256, ctx->sm_count), 256, 0, ctx->stream, b->N,
+                 b->parent, b->d_offs, b->count, dst);
     if ((st = check_launch(ctx, 1)) != DCF_OK) return st;
     if (!on_device) CU(cudaMemcpyAsync(parent, dst, N * 8, cudaMemcpyDeviceToHost, ctx->stream));
     return sync_and_check(ctx);

@@ -245,7 +245,7 @@ __global__ void k_fill_u32(long long n, uint32_t *dst, uint32_t v)
 
 void launch_fill_u32(long long n, uint32_t *dst, uint32_t v, int sm, cudaStream_t s)
 {
-    k_fill_u32<<<grid_for(n, 256, sm), 256, 0, s>>>(n, dst, v); note_launch();
+    launch_plain(k_fill_u32, grid_for(n, 256, sm), 256, 0, s, n, dst, v);
 }
 
 // Start values of the level roots' records.  The extent group's interleaved record
@@ -276,7 +276,7 @@ __global__ void k_attr_init(NodeSet ns, AttrBufs a)
 
 void launch_attr_init(const AttrBufs &a, NodeSet ns, long long n, int sm, cudaStream_t s)
 {
-    k_attr_init<<<grid_for(n, 256, sm), 256, 0, s>>>(ns, a); note_launch();
+    launch_plain(k_attr_init, grid_for(n, 256, sm), 256, 0, s, ns, a);
 }
 
 // leaves get pending = -1; nodes with exactly one child are flagged in `single`
@@ -682,12 +682,13 @@ void launch_attributes_up(const TreeView &t, AttrBufs &a, unsigned *count, int u
 {
     const int nb = grid_for(t.g.N, 256, sm);
     prof_begin(P_ATTR_UP, s);
-    k_mark_leaves<<<nb, 256, 0, s>>>(t.nodes, t.num_nodes, a.pending, a.single); note_launch();
-#define DCF_UP(G, E) k_attr_up<G, E><<<nb, 256, 0, s>>>(t.nodes, t.num_nodes, t.parent, a, up_steps, err); note_launch()
+    launch_plain(k_mark_leaves, nb, 256, 0, s, t.nodes, t.num_nodes, a.pending, a.single);
+#define DCF_UP(G, E) \
+    launch_plain(k_attr_up<G, E>, nb, 256, 0, s, t.nodes, t.num_nodes, t.parent, a, up_steps, err)
     DCF_GROUP_SWITCH(DCF_UP)
 #undef DCF_UP
     cudaMemsetAsync(count, 0, sizeof(unsigned), s);
-    k_collect_rest<<<nb, 256, 0, s>>>(t.nodes, t.num_nodes, a.pending, nullptr, count, 0u, err); note_launch();
+    launch_plain(k_collect_rest, nb, 256, 0, s, t.nodes, t.num_nodes, a.pending, nullptr, count, 0u, err);
     prof_end(P_ATTR_UP, s);
 }
 
@@ -695,7 +696,7 @@ void launch_attributes(const TreeView &t, AttrBufs &a, unsigned *count, int up_s
                        cudaStream_t s)
 {
     const int nb = grid_for(t.g.N, 256, sm);
-#define DCF_PIX(G, E) k_attr_pixels<G, E><<<nb, 256, 0, s>>>(t.gval, t.g, t.parent, t.isroot, a); note_launch()
+#define DCF_PIX(G, E) launch_plain(k_attr_pixels<G, E>, nb, 256, 0, s, t.gval, t.g, t.parent, t.isroot, a)
     prof_begin(P_ATTR_PIX, s);
     if (t.g.D == 1 && a.group <= 1 && agg_enabled()) {
         const int ntx = (t.g.W + AGG_T - 1) / AGG_T, nty = (t.g.H + AGG_T - 1) / AGG_T;
@@ -706,13 +707,12 @@ void launch_attributes(const TreeView &t, AttrBufs &a, unsigned *count, int up_s
                                      (int)agg_smem_bytes<1>());
                 attr_set = true;
             }
-            k_attr_pixels_tiled<1><<<ntx * nty, AGG_THREADS, agg_smem_bytes<1>(), s>>>(t.g, t.parent, t.isroot, a,
-                                                                                      ntx);
+            launch_plain(k_attr_pixels_tiled<1>, ntx * nty, AGG_THREADS, agg_smem_bytes<1>(), s, t.g, t.parent,
+                         t.isroot, a, ntx);
         } else {
-            k_attr_pixels_tiled<0><<<ntx * nty, AGG_THREADS, agg_smem_bytes<0>(), s>>>(t.g, t.parent, t.isroot, a,
-                                                                                      ntx);
+            launch_plain(k_attr_pixels_tiled<0>, ntx * nty, AGG_THREADS, agg_smem_bytes<0>(), s, t.g, t.parent,
+                         t.isroot, a, ntx);
         }
-        note_launch();
     } else {
         DCF_GROUP_SWITCH(DCF_PIX)
     }
@@ -743,22 +743,22 @@ static void rest_phase(const TreeView &t, AttrBufs &a, unsigned cap, bool, unsig
     cudaMemsetAsync(act, 0, 33 * sizeof(unsigned), s);
     cudaMemsetAsync(act, 1, 1, s);
     cudaMemsetAsync(count, 0, sizeof(unsigned), s);
-    k_collect_rest<<<nb, 256, 0, s>>>(t.nodes, t.num_nodes, a.pending, list, count, cap, err); note_launch();
+    launch_plain(k_collect_rest, nb, 256, 0, s, t.nodes, t.num_nodes, a.pending, list, count, cap, err);
     if (cap == 0) return;
     const int rb = grid_for(cap, 256, sm);
-    k_rest_gather<G><<<rb, 256, 0, s>>>(list, count, cap, t.parent, a.pending, a, r0, j0, err); note_launch();
-    k_rest_links<G><<<rb, 256, 0, s>>>(list, count, cap, t.parent, a.pending, j0, err); note_launch();
+    launch_plain(k_rest_gather<G>, rb, 256, 0, s, list, count, cap, t.parent, a.pending, a, r0, j0, err);
+    launch_plain(k_rest_links<G>, rb, 256, 0, s, list, count, cap, t.parent, a.pending, j0, err);
     int rounds = 0;
     while ((1u << rounds) < cap && rounds < 31) rounds++;
     RestRecs *ri = &r0, *ro = &r1;
     int *ji = j0, *jo = j1;
     for (int k = 0; k < rounds; k++) {
-        k_copy_recs<G><<<rb, 256, 0, s>>>(count, cap, *ri, *ro, a, act + k); note_launch();
-        k_jump_fold<G, E><<<rb, 256, 0, s>>>(count, cap, ji, jo, *ri, *ro, a, act + k, act + k + 1); note_launch();
+        launch_plain(k_copy_recs<G>, rb, 256, 0, s, count, cap, *ri, *ro, a, act + k);
+        launch_plain(k_jump_fold<G, E>, rb, 256, 0, s, count, cap, ji, jo, *ri, *ro, a, act + k, act + k + 1);
         RestRecs *tr = ri; ri = ro; ro = tr;
         int *tj = ji; ji = jo; jo = tj;
     }
-    k_rest_scatter<G><<<rb, 256, 0, s>>>(list, count, cap, a, r0, r1, act, rounds); note_launch();
+    launch_plain(k_rest_scatter<G>, rb, 256, 0, s, list, count, cap, a, r0, r1, act, rounds);
 }
 
 // Phase 2: R = number of nodes the walkers left (read back by the caller), scratch
@@ -800,7 +800,8 @@ void launch_node_attr(const TreeView &t, const AttrBufs &a, int attr, bool area,
                       cudaStream_t s)
 {
     int nb = grid_for(t.g.N, 256, sm);
-    k_node_attr<<<nb, 256, 0, s>>>(t.g, t.isroot, a, attr, area, t.pixdim[0], t.pixdim[1], t.pixdim[2], out); note_launch();
+    launch_plain(k_node_attr, nb, 256, 0, s, t.g, t.isroot, a, attr, area, t.pixdim[0], t.pixdim[1], t.pixdim[2],
+                 out);
 }
 
 }  // namespace dcf

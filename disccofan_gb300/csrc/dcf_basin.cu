@@ -1333,10 +1333,8 @@ static void after_basins(const ForestWork &w, const ChainOrder &c, const float *
         // up to 8128 pixels) go there directly: a cooperative launch and its barriers less, about
         // 10 us of the 129 that a call on 96 x 80 u8 took.
         const bool raw = ecap <= TAIL_EDGES && 2 * TAIL_COMPS >= (unsigned long long)comp_cap;
-        if (!raw) {
-            cudaLaunchCooperativeKernel((const void *)k_saddles, dim3(nb), dim3(SADDLE_THREADS), args, 0, s);
-            note_launch();
-        }
+        if (!raw && may_launch())
+            note_launch(cudaLaunchCooperativeKernel((const void *)k_saddles, dim3(nb), dim3(SADDLE_THREADS), args, 0, s));
         static const bool tail_set = (cudaFuncSetAttribute(k_saddles_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM), true);
         (void)tail_set;
         launch_next(k_saddles_tail, 1, TAIL_THREADS, TAIL_SMEM, s, label, ew0, ab0, ew1, ab1, comp, ctr,

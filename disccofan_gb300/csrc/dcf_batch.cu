@@ -310,9 +310,10 @@ void launch_batch_build(int dtype, const void *img, const Geom &bg, const BatchI
     batch_tile_carveout();
     cudaMemsetAsync(next, 0, sizeof(unsigned), s);
     prof_begin(P_TILE, s);
-#define DCF_TB(T)                                                                                       \
-    k_batch_tile_build<T><<<grid, TileCfg<T>::threads, tile_smem_bytes(bg.tw, bg.th, 1, TileCfg<T>::word_bytes), s>>>((const T *)img, bg, imgs, tiles, ntiles, chunk, \
-                                                          next, gval, node, err); note_launch()
+#define DCF_TB(T)                                                                                               \
+    launch_plain(k_batch_tile_build<T>, grid, TileCfg<T>::threads,                                              \
+                 tile_smem_bytes(bg.tw, bg.th, 1, TileCfg<T>::word_bytes), s, (const T *)img, bg, imgs, tiles,  \
+                 ntiles, chunk, next, gval, node, err)
     switch (dtype) {
     case U8: DCF_TB(uint8_t); break;
     case U16: DCF_TB(uint16_t); break;
@@ -327,10 +328,10 @@ void launch_batch_build(int dtype, const void *img, const Geom &bg, const BatchI
     if (seam.buckets > 0) {
         cudaMemsetAsync(seam.count, 0, 4, s);
         cudaMemsetAsync(seam.hist, 0, 4 * SEAM_BINS, s);
-        k_batch_seam_collect<<<grid_for(work, 256, sm), 256, 0, s>>>(node, bg, imgs, tiles, ntiles, seam); note_launch();
+        launch_plain(k_batch_seam_collect, grid_for(work, 256, sm), 256, 0, s, node, bg, imgs, tiles, ntiles, seam);
         launch_seam_buckets(seam, node, bg.N, bg.merge_bound, err, sm, s);
     } else {
-        k_batch_seam<<<grid_for(work, 128, sm), 128, 0, s>>>(node, bg, imgs, tiles, ntiles, err); note_launch();
+        launch_plain(k_batch_seam, grid_for(work, 128, sm), 128, 0, s, node, bg, imgs, tiles, ntiles, err);
     }
     prof_end(P_SEAM, s);
     launch_canon(node, bg, parent, isroot, num_nodes, nodes, err, sm, s);
@@ -343,7 +344,7 @@ void launch_batch_attr_pixels(const Geom &bg, const BatchImg *imgs, const BatchT
     const long long work = (long long)ntiles * bg.tw * bg.th;
     const int nb = grid_for(work, 256, sm);
     prof_begin(P_ATTR_PIX, s);
-#define DCF_BP(G, E) k_batch_attr_pixels<G, E><<<nb, 256, 0, s>>>(gval, bg, imgs, tiles, ntiles, parent, isroot, a); note_launch()
+#define DCF_BP(G, E) launch_plain(k_batch_attr_pixels<G, E>, nb, 256, 0, s, gval, bg, imgs, tiles, ntiles, parent, isroot, a)
     switch (a.group * 2 + (a.exact_g ? 1 : 0)) {
     case 0: case 1: DCF_BP(0, false); break;
     case 2: case 3: DCF_BP(1, false); break;

@@ -310,12 +310,12 @@ __global__ void k_seam_bucket(SeamEdges e, int b, unsigned long long *gnode, lon
 void launch_seam_buckets(SeamEdges &e, unsigned long long *node, long long n, long long merge_bound, unsigned *err,
                          int sm, cudaStream_t s)
 {
-    k_seam_bounds<<<1, 1024, 0, s>>>(e); note_launch();
-    k_seam_scatter<<<grid_for(e.cap, 256, sm), 256, 0, s>>>(e); note_launch();
+    launch_plain(k_seam_bounds, 1, 1024, 0, s, e);
+    launch_plain(k_seam_scatter, grid_for(e.cap, 256, sm), 256, 0, s, e);
     const int gb = grid_for(e.cap / e.buckets + 1, 128, sm);
     for (int b = 0; b < e.buckets; b++) {
-        k_seam_bucket<<<gb, 128, 0, s>>>(e, b, node, n, merge_bound > 0 ? merge_bound : MERGE_BOUND_GLOBAL, err);
-        note_launch();
+        launch_plain(k_seam_bucket, gb, 128, 0, s, e, b, node, n,
+                     merge_bound > 0 ? merge_bound : MERGE_BOUND_GLOBAL, err);
     }
 }
 
@@ -583,13 +583,13 @@ void launch_canon(unsigned long long *node, const Geom &g, int *parent, unsigned
                   unsigned long long *num_nodes, int *nodes, unsigned *err, int sm_count, cudaStream_t s)
 {
     prof_begin(P_CANON, s);
-    k_canon<<<grid_for(g.N, 256, sm_count), 256, 0, s>>>(node, g, parent, isroot, err); note_launch();
+    launch_plain(k_canon, grid_for(g.N, 256, sm_count), 256, 0, s, node, g, parent, isroot, err);
     const long long chunks = node_list_chunks(g.N);
     unsigned *counts = (unsigned *)((char *)nodes + (size_t)(4 * g.N + 255) / 256 * 256);
     const int nb = (int)(chunks < (long long)sm_count * 16 ? chunks : (long long)sm_count * 16);
-    k_nodes_count<<<nb, NL_THREADS, 0, s>>>(isroot, g.N, counts); note_launch();
-    k_nodes_scan<<<1, 1024, 0, s>>>(counts, chunks, num_nodes); note_launch();  // the node count
-    k_nodes_emit<<<nb, NL_THREADS, 0, s>>>(isroot, g.N, counts, nodes); note_launch();
+    launch_plain(k_nodes_count, nb, NL_THREADS, 0, s, isroot, g.N, counts);
+    launch_plain(k_nodes_scan, 1, 1024, 0, s, counts, chunks, num_nodes);  // the node count
+    launch_plain(k_nodes_emit, nb, NL_THREADS, 0, s, isroot, g.N, counts, nodes);
     prof_end(P_CANON, s);
 }
 
@@ -607,7 +607,7 @@ static void build_t(const BuildArgs &a, cudaStream_t s)
                             true);
     (void)carveout;
     prof_begin(P_TILE, s);
-    k_tile_build<T, MIN><<<grid, TileCfg<T>::threads, smem, s>>>(img, a.g, a.kmax, a.gval, a.node, a.err); note_launch();
+    launch_plain(k_tile_build<T, MIN>, grid, TileCfg<T>::threads, smem, s, img, a.g, a.kmax, a.gval, a.node, a.err);
     prof_end(P_TILE, s);
     prof_begin(P_SEAM, s);
     {
@@ -616,10 +616,12 @@ static void build_t(const BuildArgs &a, cudaStream_t s)
             SeamEdges e = a.seam;
             cudaMemsetAsync(e.count, 0, 4, s);
             cudaMemsetAsync(e.hist, 0, 4 * SEAM_BINS, s);
-            k_seam_collect<<<grid_for(work, 256, a.sm_count), 256, 0, s>>>(a.node, a.g, grid.x, grid.y, grid.z, e); note_launch();
+            launch_plain(k_seam_collect, grid_for(work, 256, a.sm_count), 256, 0, s, a.node, a.g, grid.x, grid.y,
+                         grid.z, e);
             launch_seam_buckets(e, a.node, a.g.N, a.g.merge_bound, a.err, a.sm_count, s);
         } else {
-            k_seam_direct<<<grid_for(work, 128, a.sm_count), 128, 0, s>>>(a.node, a.g, grid.x, grid.y, grid.z, a.err); note_launch();
+            launch_plain(k_seam_direct, grid_for(work, 128, a.sm_count), 128, 0, s, a.node, a.g, grid.x, grid.y,
+                         grid.z, a.err);
         }
     }
     prof_end(P_SEAM, s);

@@ -15,9 +15,12 @@ enum ProfId : int {
 };
 void prof_begin(int id, cudaStream_t s);
 void prof_end(int id, cudaStream_t s);
-// counts one kernel launch for the context whose API call is running on this thread
-// (dcf_ctx_launch_count); every launch site calls it right after the launch
-void note_launch();
+// Every kernel is launched between these two.  note_launch counts a launch for the context
+// whose API call is running on this thread (dcf_ctx_launch_count), or keeps why it failed;
+// from then on nothing of that call may be launched, as the kernels that follow take what
+// the missing one was to write for indices.  check_launch reports the failure.
+bool may_launch();
+void note_launch(cudaError_t e);
 // whether that call has launched a kernel before
 bool follows_launch();
 
@@ -32,6 +35,7 @@ bool follows_launch();
 template <typename... P, typename... A>
 void launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args)
 {
+    if (!may_launch()) return;
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -42,8 +46,19 @@ void launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaS
     c.stream = s;
     c.attrs = &at;
     c.numAttrs = follows_launch() ? 1 : 0;
-    cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
-    note_launch();
+    note_launch(cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...));
+}
+// an ordinary launch, of a kernel without after_previous()
+template <typename... P, typename... A>
+void launch_plain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args)
+{
+    if (!may_launch()) return;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    note_launch(cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...));
 }
 // First statement of such a kernel, in every thread: waits until all that the kernel
 // before it wrote can be read.

@@ -1,0 +1,102 @@
+"""What the library launches and allocates, on the CPU: a child process with
+fake_cudart.c in place of the CUDA runtime, which runs no kernel but refuses what the real
+one refuses (launch sizes, shared memory without the opt-in, a full device)."""
+import os
+import shutil
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+CUDA_ERROR, NOMEM = 3, 2
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    """run(code, **environment) -> (what the child printed, [(device, kernel, status) of every launch])"""
+    if shutil.which("gcc") is None or not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime_api.h")):
+        pytest.skip("needs gcc and the CUDA headers")
+    where = tmp_path_factory.mktemp("fake")
+    so = str(where / "fake_cudart.so")
+    subprocess.run(["gcc", "-O1", "-Wall", "-Werror", "-fPIC", "-shared", "-I" + os.path.join(CUDA, "include"),
+                    os.path.join(HERE, "fake_cudart.c"), "-o", so], check=True)
+
+    def child(code, **env):
+        log = str(where / "log")
+        open(log, "w").close()
+        r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(code)],
+                           env=dict(os.environ, LD_PRELOAD=so, FAKE_CUDA_LOG=log, PYTHONPATH=ROOT,
+                                    **{k: str(v) for k, v in env.items()}),
+                           capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-3000:]
+        with open(log) as f:
+            rows = [line.split() for line in f]
+        return r.stdout.split(), [(int(d), k, int(s)) for d, k, s in rows]
+
+    return child
+
+
+PRELUDE = """
+import ctypes as C, sys
+import numpy as np, disccofan_gb300 as dcf
+fail_in = C.c_int.in_dll(C.CDLL(None), "fake_fail_in")
+memory, in_use = (C.c_size_t.in_dll(C.CDLL(None), "fake_" + n) for n in ("memory", "in_use"))
+def status(f):
+    try:
+        f()
+    except dcf.DcfError as e:
+        return e.status
+    return 0
+"""
+
+
+@pytest.mark.parametrize("least", [1, 1 << 40])
+@pytest.mark.parametrize("shape,dtype,conn,rule", [((200, 230), "uint16", 8, "subtractive"), ((60, 70), "uint8", 4, "min"),
+                                                   ((20, 30, 40), "float32", 6, "direct"), ((60, 70), "uint8", 4, "max")])
+def test_nothing_is_launched_after_a_failed_launch(run, shape, dtype, conn, rule, least):
+    """Whichever launch of a call fails, it is the call's last, and the call reports it."""
+    said, rows = run(f"""
+        img = np.zeros({shape}, np.{dtype})
+        for k in range(1000):
+            ctx = dcf.Context(0)
+            fail_in.value = k
+            made = []
+            calls = [lambda: made.append(ctx.build(img, connectivity={conn}, tree_type="max", attribute=0)),
+                     lambda: made[0].set_attribute(14), lambda: made[0].filter(14, 2.0, "{rule}"),
+                     lambda: made[0].check(14), lambda: made[0].pattern_spectrum(14, np.float32([0, 1, 2]))]
+            for call in calls:
+                st = status(call)
+                if st:
+                    assert st == {CUDA_ERROR} and ctx.launches == k, (k, st, ctx.launches)
+                    break
+            else:
+                break
+        print(k)
+        """, DCF_BASIN_MIN=least)
+    assert int(said[0]) > 10
+    assert sum(s != 0 for _, _, s in rows) == int(said[0])
+
+
+def test_launches_of_a_batch_stop_at_a_failed_one(run):
+    for least in (1, 1 << 40):
+        said, rows = run(f"""
+            shapes = [(40, 50), (70, 33)]
+            pix = np.zeros(40 * 50 + 70 * 33, np.float32)
+            lv = np.float32([0, 1, 2])
+            for k in range(1000):
+                ctx = dcf.Context(0)
+                b = ctx.batch(shapes, np.float32, connectivity=8, attribute=13)
+                fail_in.value = k
+                st = status(lambda: b.run(pix, filter_attr=0, lam=3.0, spectrum=(13, lv, 0, lv), use_graph=False))
+                b.close()
+                if not st:
+                    break
+                assert st == {CUDA_ERROR} and ctx.launches == k, (k, st, ctx.launches)
+            print(k)
+            """, DCF_BASIN_MIN=least)
+        assert int(said[0]) > 10
+        assert sum(s != 0 for _, _, s in rows) == int(said[0])
