@@ -547,19 +547,11 @@ static cudaError_t attr_zero(const AttrBufs &a, const int *nodes, const unsigned
     return cudaGetLastError();
 }
 
-// allocate and accumulate the records of attr_idx's group
-// need_grey: the inertia group must also accumulate the grey-weighted sums (the
-// tree file's weighted centroids); its attributes 13-17 do not read them
-static dcf_status compute_attributes(dcf_ctx *ctx, dcf_tree *t, int attr_idx, bool need_grey = false)
+// allocate and accumulate the records of a group, in place of those there were
+static dcf_status fill_attributes(dcf_ctx *ctx, dcf_tree *t, int group, bool need_grey)
 {
-    const int group = ATTR_GROUP[attr_idx];
-    if (t->attr_mem && t->attr.group == group && (!need_grey || t->attr.grey)) {
-        t->attr_idx = attr_idx;
-        return DCF_OK;
-    }
-    dcf_status st = refuse_capture(ctx);
-    if (st != DCF_OK) return st;
     free_attr(t);
+    dcf_status st;
     const size_t N = (size_t)t->g.N;
     CU(dmalloc_async(ctx, &t->attr_mem, attr_bytes(group, t->g.D > 1, need_grey, N), ctx->stream));
     AttrBufs &a = t->attr;
@@ -567,10 +559,7 @@ static dcf_status compute_attributes(dcf_ctx *ctx, dcf_tree *t, int attr_idx, bo
     void *ws = nullptr;
     if (t->chains.n) {
         st = scratch(ctx, 8, chain_attr_bytes(a, t->g.N, t->chain_cap), &ws);
-        if (st != DCF_OK && !(st == DCF_ERR_NOMEM && ctx->fail_alloc < 0)) {
-            free_attr(t);
-            return st;
-        }
+        if (st != DCF_OK && !(st == DCF_ERR_NOMEM && ctx->fail_alloc < 0)) return st;
     }
     // without memory for the running sums the records are folded along the parents, which
     // needs less of it
@@ -585,7 +574,6 @@ static dcf_status compute_attributes(dcf_ctx *ctx, dcf_tree *t, int attr_idx, bo
         ca.err = ctx->d_err;
         ca.sm_count = ctx->sm_count;
         launch_chain_attr(ca, ctx->stream);
-        t->attr_idx = attr_idx;
         return check_launch(ctx, 4);
     }
     cudaGetLastError();  // a failed allocation must not pass for a failed launch
@@ -599,13 +587,26 @@ static dcf_status compute_attributes(dcf_ctx *ctx, dcf_tree *t, int attr_idx, bo
     CU(cudaStreamSynchronize(ctx->stream));
     if (R > 0) {
         st = scratch(ctx, 8, attr_rest_bytes(group, R), &ws);
-        if (st != DCF_OK) {
-            free_attr(t);
+        if (st != DCF_OK) return st;
+        launch_attributes_rest(view_of(t), a, R, count, ws, ctx->d_err, ctx->sm_count, ctx->stream);
+        return check_launch(ctx, 4);
+    }
+    return DCF_OK;
+}
+
+// the records of attr_idx's group
+// need_grey: the inertia group must also accumulate the grey-weighted sums (the
+// tree file's weighted centroids); its attributes 13-17 do not read them
+static dcf_status compute_attributes(dcf_ctx *ctx, dcf_tree *t, int attr_idx, bool need_grey = false)
+{
+    const int group = ATTR_GROUP[attr_idx];
+    if (!(t->attr_mem && t->attr.group == group && (!need_grey || t->attr.grey))) {
+        dcf_status st = refuse_capture(ctx);
+        if (st != DCF_OK) return st;
+        if ((st = fill_attributes(ctx, t, group, need_grey)) != DCF_OK) {
+            free_attr(t);  // a later call must not take unwritten records for the group's
             return st;
         }
-        launch_attributes_rest(view_of(t), a, R, count, ws, ctx->d_err, ctx->sm_count, ctx->stream);
-        st = check_launch(ctx, 4);
-        if (st != DCF_OK) return st;
     }
     t->attr_idx = attr_idx;
     return DCF_OK;

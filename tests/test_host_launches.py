@@ -12,7 +12,7 @@ import pytest
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-CUDA_ERROR, NOMEM = 3, 2
+NOMEM, CUDA_ERROR, STATE = 2, 3, 6
 
 
 @pytest.fixture(scope="module")
@@ -100,3 +100,27 @@ def test_launches_of_a_batch_stop_at_a_failed_one(run):
             """, DCF_BASIN_MIN=least)
         assert int(said[0]) > 10
         assert sum(s != 0 for _, _, s in rows) == int(said[0])
+
+
+@pytest.mark.parametrize("least", [1, 1 << 40])
+def test_records_of_a_failed_attribute_pass_are_not_kept(run, least):
+    """After a set_attribute that failed, whichever launch of it did, the tree has no
+    attributes, and the next one computes them."""
+    said, _ = run(f"""
+        ctx = dcf.Context(0)
+        t = ctx.build(np.zeros((50, 60), np.uint16), connectivity=8, tree_type="max", attribute=0)
+        before = ctx.launches
+        t.set_attribute(14)
+        whole = ctx.launches - before
+        t.set_attribute(0)
+        for k in range(whole):
+            fail_in.value = k
+            assert status(lambda: t.set_attribute(14)) == {CUDA_ERROR}
+            assert status(lambda: t.filter(14, 2.0)) == {STATE}
+            before = ctx.launches
+            t.set_attribute(14)
+            assert ctx.launches - before == whole
+            t.set_attribute(0)
+        print(whole)
+        """, DCF_BASIN_MIN=least)
+    assert int(said[0]) >= 4
