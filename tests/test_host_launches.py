@@ -109,6 +109,8 @@ def test_records_of_a_failed_attribute_pass_are_not_kept(run, least):
     said, _ = run(f"""
         ctx = dcf.Context(0)
         t = ctx.build(np.zeros((50, 60), np.uint16), connectivity=8, tree_type="max", attribute=0)
+        out = np.zeros(3000, np.float32)
+        use = lambda: ctx.lib.dcf_filter(ctx.h, t.h, 14, 0, 2.0, 0, out.ctypes.data, 0)
         before = ctx.launches
         t.set_attribute(14)
         whole = ctx.launches - before
@@ -116,10 +118,10 @@ def test_records_of_a_failed_attribute_pass_are_not_kept(run, least):
         for k in range(whole):
             fail_in.value = k
             assert status(lambda: t.set_attribute(14)) == {CUDA_ERROR}
-            assert status(lambda: t.filter(14, 2.0)) == {STATE}
+            assert use() == {STATE}
             before = ctx.launches
             t.set_attribute(14)
-            assert ctx.launches - before == whole
+            assert ctx.launches - before == whole and use() == 0
             t.set_attribute(0)
         print(whole)
         """, DCF_BASIN_MIN=least)
