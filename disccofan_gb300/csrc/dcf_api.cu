@@ -357,6 +357,12 @@ dcf_status dcf_ctx_create(int device, void *cuda_stream, dcf_ctx **out)
         int v = atoi(e);
         if (v >= 0 && v < (1 << 20)) ctx->up_steps = v;
     }
+    if (basin_opt_in() != cudaSuccess || attr_opt_in() != cudaSuccess) {
+        cudaGetLastError();
+        if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
+        delete ctx;
+        return DCF_ERR_CUDA;
+    }
     // keep freed tree buffers in the device's default pool: repeated builds then
     // allocate stream-ordered without cudaMalloc's cost or its implicit sync
     cudaMemPool_t pool;

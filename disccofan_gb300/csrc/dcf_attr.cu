@@ -692,6 +692,12 @@ void launch_attributes_up(const TreeView &t, AttrBufs &a, unsigned *count, int u
     prof_end(P_ATTR_UP, s);
 }
 
+cudaError_t attr_opt_in()
+{
+    return cudaFuncSetAttribute(k_attr_pixels_tiled<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)agg_smem_bytes<1>());
+}
+
 void launch_attributes(const TreeView &t, AttrBufs &a, unsigned *count, int up_steps, unsigned *err, int sm,
                        cudaStream_t s)
 {
@@ -701,12 +707,6 @@ void launch_attributes(const TreeView &t, AttrBufs &a, unsigned *count, int up_s
     if (t.g.D == 1 && a.group <= 1 && agg_enabled()) {
         const int ntx = (t.g.W + AGG_T - 1) / AGG_T, nty = (t.g.H + AGG_T - 1) / AGG_T;
         if (a.group == 1) {
-            static bool attr_set = false;  // opt in to more than 48 KB of dynamic shared memory, once
-            if (!attr_set) {
-                cudaFuncSetAttribute(k_attr_pixels_tiled<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)agg_smem_bytes<1>());
-                attr_set = true;
-            }
             launch_plain(k_attr_pixels_tiled<1>, ntx * nty, AGG_THREADS, agg_smem_bytes<1>(), s, t.g, t.parent,
                          t.isroot, a, ntx);
         } else {

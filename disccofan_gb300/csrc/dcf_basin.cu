@@ -1309,6 +1309,13 @@ ForestWork forest_carve(void *mem, int conn, long long n, long long basin_cap, s
     return w;
 }
 
+cudaError_t basin_opt_in()
+{
+    const cudaError_t e = cudaFuncSetAttribute(k_saddles_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_rs_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SMEM);
+}
+
 template <int KB>
 static void after_basins(const ForestWork &w, const ChainOrder &c, const float *gval, long long n, long long comp_cap, long long max_rounds,
                          int *parent, unsigned *err, int sm, cudaStream_t s)
@@ -1335,8 +1342,6 @@ static void after_basins(const ForestWork &w, const ChainOrder &c, const float *
         const bool raw = ecap <= TAIL_EDGES && 2 * TAIL_COMPS >= (unsigned long long)comp_cap;
         if (!raw && may_launch())
             note_launch(cudaLaunchCooperativeKernel((const void *)k_saddles, dim3(nb), dim3(SADDLE_THREADS), args, 0, s));
-        static const bool tail_set = (cudaFuncSetAttribute(k_saddles_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM), true);
-        (void)tail_set;
         launch_next(k_saddles_tail, 1, TAIL_THREADS, TAIL_SMEM, s, label, ew0, ab0, ew1, ab1, comp, ctr,
                     raw ? ecap : 0u, max_rounds, err);
     }
@@ -1348,8 +1353,6 @@ static void after_basins(const ForestWork &w, const ChainOrder &c, const float *
     const int cb_blocks = grid_for(comp_cap, 256, sm);
     prof_end(P_SADDLES, s);
     prof_begin(P_SORT, s);
-    static const bool smem_set = (cudaFuncSetAttribute(k_rs_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SMEM), true);
-    (void)smem_set;
     int cb = 0;
     while ((1LL << cb) < comp_cap) cb++;
     const int passes = (KB + cb + 7) / 8, nblk = (int)rs_blocks(n);

@@ -64,6 +64,11 @@ void launch_plain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cuda
 // before it wrote can be read.
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Opt-ins of a unit's kernels to more than 48 KB of dynamic shared memory.  They hold for the
+// device that is current and go with a device reset, so every context asks for its own.
+cudaError_t basin_opt_in();
+cudaError_t attr_opt_in();
+
 constexpr int TILE_THREADS = 256;        // tile build CTAs with 64-bit shared node words (u32/f32)
 constexpr int TILE_THREADS_NARROW = 128; // with 32-bit words (u8/u16): more tiles resident per SM
 constexpr int TILE_MAX_PIX = 4096;             // largest build tile (16-bit local indices)

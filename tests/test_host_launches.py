@@ -126,3 +126,25 @@ def test_records_of_a_failed_attribute_pass_are_not_kept(run, least):
         print(whole)
         """, DCF_BASIN_MIN=least)
     assert int(said[0]) >= 4
+
+
+@pytest.mark.parametrize("least", [1, 1 << 40])
+def test_contexts_on_two_devices_of_one_process(run, least):
+    """Opt-ins to more than 48 KB of shared memory hold for one device: a context on a
+    second one needs its own, and so does one made after the device was reset."""
+    said, rows = run("""
+        def everything(device):
+            ctx = dcf.Context(device)
+            for attr in (0, 18, 14):
+                t = ctx.build(np.zeros((300, 410), np.uint16), connectivity=8, tree_type="max", attribute=attr)
+                t.filter(attr, 2.0)
+                t.pattern_spectrum(attr, np.float32([0, 1, 2]))
+            b = ctx.batch([(40, 50), (70, 33)], np.float32, connectivity=8, attribute=13)
+            b.run(np.zeros(40 * 50 + 70 * 33, np.float32), filter_attr=0, lam=3.0, use_graph=False)
+        everything(0)
+        everything(1)
+        C.CDLL(None).fake_reset()
+        everything(1)
+        """, DCF_BASIN_MIN=least)
+    assert {d for d, _, _ in rows} == {0, 1}
+    assert not [r for r in rows if r[2]]
