@@ -118,9 +118,11 @@ k_basins(const T *__restrict__ img, Geom g, const BatchImg *__restrict__ imgs, c
         x0 = tl.x0;
         y0 = tl.y0;
     } else {
-        x0 = blockIdx.x * BT::X;
-        y0 = blockIdx.y * BT::Y;
-        z0 = blockIdx.z * BT::Z;
+        // tiles x fastest in a 1-D grid: one has room for 65535 rows or slices only
+        const unsigned tx = (W + BT::X - 1) / BT::X, ty = (H + BT::Y - 1) / BT::Y, row = blockIdx.x / tx;
+        x0 = (int)(blockIdx.x - row * tx) * BT::X;
+        y0 = (int)(row % ty) * BT::Y;
+        z0 = (int)(row / ty) * BT::Z;
     }
     const int D = BT::flat ? 1 : g.D;
     const long long WH = (long long)W * H;
@@ -1398,7 +1400,8 @@ template <typename T, bool MIN, int CONN, bool BATCH>
 static void basins(const ForestArgs &a, cudaStream_t s)
 {
     using BT = BasinTile<CONN>;
-    const dim3 grid = BATCH ? dim3(a.ntiles) : dim3((a.g.W + BT::X - 1) / BT::X, (a.g.H + BT::Y - 1) / BT::Y, (a.g.D + BT::Z - 1) / BT::Z);
+    auto tiles = [](int side, int tile) { return (unsigned)((side + tile - 1) / tile); };
+    const unsigned grid = BATCH ? a.ntiles : tiles(a.g.W, BT::X) * tiles(a.g.H, BT::Y) * tiles(a.g.D, BT::Z);
     launch_next(k_basins<T, MIN, CONN, BATCH>, grid, BASIN_THREADS, 0, s, (const T *)a.img, a.g, a.imgs, a.tiles,
                 a.kmax, a.gval, a.w.label, a.w.ew[0], a.w.eab[0], a.w.ctr, (unsigned)a.w.ecap, a.err);
 }

@@ -227,3 +227,25 @@ def test_large_images_same_as_merging_build(builds, shape, dtype):
         got, want = (x.build(img, connectivity=4, tree_type=tree, attribute=0) for x in builds)
         assert np.array_equal(got.parent(), want.parent())
         assert np.array_equal(got.filter(0, 9.0), want.filter(0, 9.0))
+
+
+@pytest.mark.gpu
+def test_more_rows_and_slices_than_a_grid_has(builds):
+    """Pixels in one column or one line of slices are the same graph as in one row: the same
+    parents, from tiles whose numbers go beyond 65535 rows or slices of them."""
+    n = 65536 * 32 + 77
+    row = (np.random.default_rng(6).integers(0, 9, n) + np.arange(n) // 50_000).astype(np.uint8)
+    def parents(img, conn):
+        t = builds[0].build(img, connectivity=conn, tree_type="max", attribute=0)
+        p = t.parent()
+        t.close()
+        return p
+    assert np.array_equal(parents(row.reshape(n, 1), 4), parents(row.reshape(1, n), 4))
+    m = 65536 * 8 + 33
+    want = parents(row[:m].reshape(1, m), 4)
+    assert np.array_equal(parents(row[:m].reshape(m, 1, 1), 6), want)
+    assert np.array_equal(parents(row[:m].reshape(m, 1, 1), 26), want)
+    # two slices of one column each: the columns' other neighbours are m pixels apart
+    two = row[:2 * (m // 2)]
+    got, flat = parents(two.reshape(2, -1, 1), 6), parents(two.reshape(2, -1), 4)
+    assert np.array_equal(got, flat)

@@ -148,3 +148,24 @@ def test_contexts_on_two_devices_of_one_process(run, least):
         """, DCF_BASIN_MIN=least)
     assert {d for d, _, _ in rows} == {0, 1}
     assert not [r for r in rows if r[2]]
+
+
+@pytest.mark.parametrize("shape,conn", [((2_097_121, 1), 4), ((2_097_153, 2), 8), ((524_281, 1, 1), 6),
+                                        ((524_289, 2, 1), 26), ((2, 1_048_561, 1), 6)])
+def test_tall_images_are_built(run, shape, conn):
+    """Rows and slices beyond 65535 tiles of them: no launch is refused."""
+    said, rows = run(f"""
+        ctx = dcf.Context(0)
+        ctx.build(np.zeros({shape}, np.uint8), connectivity={conn}, tree_type="max", attribute=0)
+        """)
+    assert len(rows) > 15 and not [r for r in rows if r[2]]
+
+
+def test_merging_build_refuses_what_its_launch_cannot_hold(run):
+    """The merging build's tiles are a 3-D grid: taller images end at its tile kernel."""
+    said, rows = run("""
+        ctx = dcf.Context(0)
+        print(status(lambda: ctx.build(np.zeros((2_097_121, 1), np.uint8), connectivity=4, tree_type="max", attribute=0)))
+        """, DCF_BASIN_MIN=1 << 40)
+    assert said == [str(CUDA_ERROR)] and [r[2] != 0 for r in rows] == [False] * (len(rows) - 1) + [True]
+    assert "k_tile_build" in rows[-1][1]
