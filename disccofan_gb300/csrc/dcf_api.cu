@@ -357,7 +357,7 @@ dcf_status dcf_ctx_create(int device, void *cuda_stream, dcf_ctx **out)
         int v = atoi(e);
         if (v >= 0 && v < (1 << 20)) ctx->up_steps = v;
     }
-    if (basin_opt_in() != cudaSuccess || attr_opt_in() != cudaSuccess) {
+    if (basin_opt_in() != cudaSuccess || attr_opt_in() != cudaSuccess || ops_opt_in() != cudaSuccess) {
         cudaGetLastError();
         if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
         delete ctx;

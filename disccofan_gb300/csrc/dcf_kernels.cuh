@@ -68,6 +68,7 @@ __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.
 // device that is current and go with a device reset, so every context asks for its own.
 cudaError_t basin_opt_in();
 cudaError_t attr_opt_in();
+cudaError_t ops_opt_in();
 
 constexpr int TILE_THREADS = 256;        // tile build CTAs with 64-bit shared node words (u32/f32)
 constexpr int TILE_THREADS_NARROW = 128; // with 32-bit words (u8/u16): more tiles resident per SM

@@ -2,8 +2,9 @@
  * Device memory is host memory, copies and fills work, kernels are not run; every launch
  * is checked against what the real runtime refuses (grid and block sizes, dynamic shared
  * memory beyond 48 KB without the function's opt-in on the current device) and written to
- * the file FAKE_CUDA_LOG as "<device> <kernel> <status>".  fake_fail_in: launches until one
- * fails (-1: none does); fake_memory: bytes the device has; fake_in_use: bytes taken. */
+ * the file FAKE_CUDA_LOG as "<device> <kernel> <status> <dynamic shared memory> <opt-in>".
+ * fake_fail_in: launches until one fails (-1: none does); fake_memory: bytes the device has;
+ * fake_in_use: bytes taken. */
 #define _GNU_SOURCE
 #include <cuda_runtime_api.h>
 #include <stdint.h>
@@ -83,7 +84,7 @@ static cudaError_t launch(const void *fn, dim3 g, dim3 b, size_t smem)
     else if (fake_fail_in == 0) e = cudaErrorLaunchOutOfResources;
     if (fake_fail_in >= 0) fake_fail_in--;
     if (!log) log = fopen(getenv("FAKE_CUDA_LOG"), "w");
-    fprintf(log, "%d %s %d\n", device, f < 0 ? "?" : funcs[f].name, (int)e);
+    fprintf(log, "%d %s %d %zu %d\n", device, f < 0 ? "?" : funcs[f].name, (int)e, smem, f < 0 ? 0 : funcs[f].smem[device]);
     fflush(log);
     return out(e);
 }

@@ -17,7 +17,8 @@ NOMEM, CUDA_ERROR, STATE = 2, 3, 6
 
 @pytest.fixture(scope="module")
 def run(tmp_path_factory):
-    """run(code, **environment) -> (what the child printed, [(device, kernel, status) of every launch])"""
+    """run(code, **environment) -> (what the child printed, [(device, kernel, status,
+    dynamic shared memory, opt-in) of every launch])"""
     if shutil.which("gcc") is None or not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime_api.h")):
         pytest.skip("needs gcc and the CUDA headers")
     where = tmp_path_factory.mktemp("fake")
@@ -35,7 +36,7 @@ def run(tmp_path_factory):
         assert r.returncode == 0, r.stderr[-3000:]
         with open(log) as f:
             rows = [line.split() for line in f]
-        return r.stdout.split(), [(int(d), k, int(s)) for d, k, s in rows]
+        return r.stdout.split(), [(int(r[0]), r[1], *map(int, r[2:])) for r in rows]
 
     return child
 
@@ -78,7 +79,7 @@ def test_nothing_is_launched_after_a_failed_launch(run, shape, dtype, conn, rule
         print(k)
         """, DCF_BASIN_MIN=least)
     assert int(said[0]) > 10
-    assert sum(s != 0 for _, _, s in rows) == int(said[0])
+    assert sum(s != 0 for _, _, s, *_ in rows) == int(said[0])
 
 
 def test_launches_of_a_batch_stop_at_a_failed_one(run):
@@ -99,7 +100,7 @@ def test_launches_of_a_batch_stop_at_a_failed_one(run):
             print(k)
             """, DCF_BASIN_MIN=least)
         assert int(said[0]) > 10
-        assert sum(s != 0 for _, _, s in rows) == int(said[0])
+        assert sum(s != 0 for _, _, s, *_ in rows) == int(said[0])
 
 
 @pytest.mark.parametrize("least", [1, 1 << 40])
@@ -146,7 +147,7 @@ def test_contexts_on_two_devices_of_one_process(run, least):
         C.CDLL(None).fake_reset()
         everything(1)
         """, DCF_BASIN_MIN=least)
-    assert {d for d, _, _ in rows} == {0, 1}
+    assert {r[0] for r in rows} == {0, 1}
     assert not [r for r in rows if r[2]]
 
 
@@ -169,3 +170,18 @@ def test_merging_build_refuses_what_its_launch_cannot_hold(run):
         """, DCF_BASIN_MIN=1 << 40)
     assert said == [str(CUDA_ERROR)] and [r[2] != 0 for r in rows] == [False] * (len(rows) - 1) + [True]
     assert "k_tile_build" in rows[-1][1]
+
+
+@pytest.mark.parametrize("n", [1, 441, 3584, 3585, 4096, 4097])
+@pytest.mark.parametrize("dtype", ["uint16", "float32"])
+def test_spectra_have_room_beside_static_shared_memory(run, dtype, n):
+    """k_spectrum<true> has its thresholds in static shared memory (6144 bytes): with the
+    histogram that may be more than a kernel gets without an opt-in."""
+    said, rows = run(f"""
+        ctx = dcf.Context(0)
+        t = ctx.build(np.zeros((50, 60), np.{dtype}), connectivity=8, tree_type="max", attribute=18)
+        t.pattern_spectrum(18, np.arange({n}, dtype=np.float32))
+        """)
+    device, name, status, dynamic, opted = rows[-1]
+    assert "k_spectrum" in name and status == 0
+    assert opted or dynamic + 6144 <= 48 * 1024
