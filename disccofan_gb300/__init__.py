@@ -481,6 +481,9 @@ class Tree:
         return self._shape(a)
 
     def check(self, attribute: int, out=None):
+        """tree_attribute_check: every pixel's node's attribute as float32.  It is
+        float32(node_attribute), but attributes 13, 14 and 17 of planar nodes are rounded
+        from exact moments (include/dcf.h), so the two may differ in the last places."""
         self._ensure_group(attribute)
         a, p, dev = self._out(np.float32, out)
         with self.ctx.ordered(a):

@@ -144,7 +144,12 @@ dcf_status dcf_filter(dcf_ctx *ctx, dcf_tree *tree, int attr_idx, int rule, doub
  * back.  Other types: DCF_ERR_INVALID. */
 dcf_status dcf_filter_as(dcf_ctx *ctx, dcf_tree *tree, int attr_idx, int rule, double lambda, int extract,
                          int out_dtype, void *out, int on_device);
-/* out[p] = (float) attribute of p's node. */
+/* out[p] = the attribute of p's node as a float.  That is (float) dcf_node_attribute,
+ * except for trace, elongation and non-compactness (13, 14, 17) of planar nodes (of
+ * 2-D images, or inside a volume's first slice) with unit pixels, sides up to 65536
+ * and an elongation below about 1000: there it lies within half a float ulp plus 2^-30
+ * of the attribute's true value, while the double readout, which subtracts large sums,
+ * may be a few float ulps off on small nodes far from the origin. */
 dcf_status dcf_attribute_check(dcf_ctx *ctx, dcf_tree *tree, int attr_idx, float *out, int on_device);
 /* Differential morphological profile: for each lvec[i+1], i < num_lambdas-1,
  * out[i*N + p] = gval - filter(lvec[i+1]). */
