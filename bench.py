@@ -539,10 +539,9 @@ def run_batch(args, ctx, stream):
     spec = (13, l_tr, 0, l_ar)
     b = ctx.batch(shapes, np.float32, connectivity=8, attribute=13)
     spectra = torch.empty((len(shapes), l_ar.size, l_tr.size), dtype=torch.float64, device="cuda")
-    # the schedule is tuned on the batch itself (default), or on a sample batch of the
-    # first tune_n cutouts applied to the whole batch.  A small sample misleads: its
-    # seam merge is bound by the longest chain walks, the whole batch's by contention,
-    # so they prefer different merge orders.
+    # the tuner runs on the batch itself (default), or on a sample batch of the first
+    # tune_n cutouts, whose schedule the whole batch then takes.  It has a choice to make
+    # only for batches that merge tiles; otherwise it reports the build's time.
     tune_n = min(len(shapes), args.tune_sample)
     t0 = time.perf_counter()
     tune_ms = None

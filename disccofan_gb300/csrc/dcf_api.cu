@@ -1967,7 +1967,7 @@ dcf_status dcf_batch_autotune(dcf_ctx *ctx, dcf_batch *b, const void *pixels, in
     CU(cudaEventCreate(&e1));
     const bool prof = ctx->prof_on;
     ctx->prof_on = false;
-    // time the build phase (queue reset, persistent tile kernel, seams, canonical form)
+    // time the build phase
     auto time_build = [&](double *ms) -> dcf_status {
         std::vector<float> t;
         for (int r = 0; r <= repeats; r++) {  // the first pass warms up
@@ -1985,6 +1985,20 @@ dcf_status dcf_batch_autotune(dcf_ctx *ctx, dcf_batch *b, const void *pixels, in
         *ms = t[t.size() / 2];
         return DCF_OK;
     };
+    auto finish = [&](dcf_status st, double ms) -> dcf_status {
+        ctx->prof_on = prof;
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        if (st != DCF_OK) return st;
+        b->valid = false;  // the timed runs leave no usable state
+        if (best_ms) *best_ms = ms;
+        return batch_check(ctx, b, nullptr);
+    };
+    if (b->forest_mem) {  // nothing below reaches the basin build: one time, no choice to make
+        double ms = 0.0;
+        const dcf_status st = time_build(&ms);
+        return finish(st, ms);
+    }
     struct Cand {
         int tw, th, ctas, chunk;
     };
@@ -2059,13 +2073,7 @@ dcf_status dcf_batch_autotune(dcf_ctx *ctx, dcf_batch *b, const void *pixels, in
         b->ops = keep;
         b->rest_cap = 0;
     }
-    ctx->prof_on = prof;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    if (st != DCF_OK) return st;
-    b->valid = false;  // the timed runs leave no usable state
-    if (best_ms) *best_ms = best_t;
-    return batch_check(ctx, b, nullptr);
+    return finish(st, best_t);
 }
 
 dcf_status dcf_batch_run(dcf_ctx *ctx, dcf_batch *b, const void *pixels, int pixels_on_device, const dcf_op_set *ops,

@@ -225,9 +225,11 @@ dcf_status dcf_batch_set_schedule(dcf_ctx *ctx, dcf_batch *batch, int tile_w, in
  * edges are merged in (0 = all at once; at most 256); up_steps = bottom-up fold
  * steps per walker before the remaining nodes are finished by pointer jumping. */
 dcf_status dcf_batch_set_merge(dcf_ctx *ctx, dcf_batch *batch, int seam_buckets, int up_steps);
-/* Time, on these pixels, the build over tile shapes, then CTAs per SM and queue
- * chunk for the best shape, then seam buckets, then build + attributes over
- * bottom-up steps; keep the fastest of each.  Leaves no valid trees. */
+/* Batches that merge tiles: time, on these pixels, the build over tile shapes, then
+ * CTAs per SM and queue chunk for the best shape, then seam buckets, then build +
+ * attributes over bottom-up steps; keep the fastest of each.  Other batches' builds
+ * depend on none of these: the build is timed and the schedule stays as it is.
+ * Leaves no valid trees. */
 dcf_status dcf_batch_autotune(dcf_ctx *ctx, dcf_batch *batch, const void *pixels, int on_device, int repeats,
                               double *best_ms);
 /* Build every cutout's tree and attributes, then the requested operations:

@@ -185,3 +185,25 @@ def test_spectra_have_room_beside_static_shared_memory(run, dtype, n):
     device, name, status, dynamic, opted = rows[-1]
     assert "k_spectrum" in name and status == 0
     assert opted or dynamic + 6144 <= 48 * 1024
+
+
+def test_autotuner_leaves_what_it_cannot_measure(run):
+    """Nothing of a basin batch's build depends on the schedule: the tuner times the build
+    once and keeps the schedule, which governs the spectrum's tile walk.  A merging batch
+    is tuned as ever."""
+    code = """
+        ctx = dcf.Context(0)
+        b = ctx.batch([(300, 410), (70, 33)], np.float32, connectivity=8, attribute=13)
+        pix = np.zeros(300 * 410 + 70 * 33, np.float32)
+        b.set_schedule((128, 32), 1, 2)
+        b.set_merge(seam_buckets=8, up_steps=77)
+        before = b.info()
+        ms = b.autotune(pix, repeats=2)
+        after = b.info()
+        print(ms, int(all(before[k] == after[k] for k in ("tile", "ctas_per_sm", "chunk", "seam_buckets", "up_steps"))))
+        """
+    said, rows = run(code)
+    assert said == ["1.0", "1"]
+    assert sum("k_basins" in r[1] for r in rows) == 3  # a warm-up and two repeats
+    said, rows = run(code, DCF_BASIN_MIN=1 << 40)
+    assert float(said[0]) == 1.0 and sum("k_batch_tile_build" in r[1] for r in rows) > 10
