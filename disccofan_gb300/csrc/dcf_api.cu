@@ -1132,15 +1132,22 @@ static dcf_status run_filter(dcf_ctx *ctx, dcf_tree *t, int attr_idx, int rule, 
     FilterWork w{};
     void *p;
     dcf_status st;
-    // min rule, and subtractive rule on integer levels: along the chain order
-    const bool path = t->chains.n && (rule == 1 || (rule == 3 && (t->dtype == U8 || t->dtype == U16)));
+    // min rule, and subtractive rule on integer levels: along the chain order, or, where a
+    // device has no room for that scratch, by the flags and pointer jumping
+    bool path = t->chains.n && (rule == 1 || (rule == 3 && (t->dtype == U8 || t->dtype == U16)));
     if (path) {
-        if ((st = scratch(ctx, 1, chain_filter_bytes(t->g.N, t->chain_cap), &w.chain_mem)) != DCF_OK) return st;
-        if ((st = scratch(ctx, 5, N * 8, &p)) != DCF_OK) return st;
-        w.acc = (double *)p;
-    } else if ((st = direct_scratch(ctx, t, rule, w)) != DCF_OK) {
-        return st;
+        st = scratch(ctx, 1, chain_filter_bytes(t->g.N, t->chain_cap), &w.chain_mem);
+        if (st == DCF_OK && (st = scratch(ctx, 5, N * 8, &p)) == DCF_OK) w.acc = (double *)p;
+        if (st != DCF_OK && !(st == DCF_ERR_NOMEM && ctx->fail_alloc < 0)) return st;
+        if (st != DCF_OK) {
+            cudaGetLastError();
+            cudaFree(ctx->scratch[1].p);  // it holds more than the flags need
+            ctx->scratch[1] = DevBuf();
+            path = false;
+            w.chain_mem = nullptr;
+        }
     }
+    if (!path && (st = direct_scratch(ctx, t, rule, w)) != DCF_OK) return st;
     if (rule == 2) {
         if ((st = scratch(ctx, 3, N * 4, &p)) != DCF_OK) return st;
         w.kept = (unsigned *)p;

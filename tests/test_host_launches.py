@@ -207,3 +207,20 @@ def test_autotuner_leaves_what_it_cannot_measure(run):
     assert sum("k_basins" in r[1] for r in rows) == 3  # a warm-up and two repeats
     said, rows = run(code, DCF_BASIN_MIN=1 << 40)
     assert float(said[0]) == 1.0 and sum("k_batch_tile_build" in r[1] for r in rows) > 10
+
+
+def test_min_rule_without_room_for_the_chains_scratch(run):
+    """The min rule along the chains wants 8 bytes a pixel at once and a value a chain; with
+    less free than that, but enough for what the general path still lacks after a max filter
+    (4 + 4 bytes a pixel), it takes that one."""
+    said, rows = run("""
+        n = 400 * 500
+        ctx = dcf.Context(0)
+        t = ctx.build(np.zeros((400, 500), np.uint16), connectivity=4, tree_type="max", attribute=0)
+        memory.value = in_use.value  # full: the next allocation takes the build's scratch back
+        t.filter(0, 5.0, "max")
+        memory.value = in_use.value + 8 * n + 4096
+        print(status(lambda: t.filter(0, 5.0, "min")))
+        """)
+    assert said == ["0"]
+    assert any("k_jump_last" in r[1] for r in rows)
