@@ -68,8 +68,9 @@ struct dcf_ctx {
     long long allocs = 0;
     cudaEvent_t input_read = nullptr; // the last build has read its input
     bool forest_busy = false;         // a build is being launched on scratch[FOREST_SLOT]
-    std::mutex trees_mu;
+    std::mutex trees_mu;              // trees and batches
     std::set<dcf_tree *> trees;       // live trees; orphaned (stream cleared) when the context goes
+    std::set<dcf_batch *> batches;    // live batches, whose basin scratch can be given back
     DevBuf scratch[16];               // reusable work buffers (filter, spectra, attributes, seams)
     DevBuf stage;                     // the image staged by dcf_image_stage (stream-ordered pool memory)
     bool prof_on = false;
@@ -199,24 +200,37 @@ static bool alloc_refused(dcf_ctx *c)
     return c->allocs++ == c->fail_alloc;
 }
 static bool device_full(const dcf_ctx *c) { return c && c->allocs == c->short_alloc + 1; }
-// The basin build's scratch is the largest buffer a context keeps, and builds can do
-// without it: when the device is out of memory it is given back and the allocation
-// tried again (not while a build still has launches or copies on it to issue).
-static bool give_back_forest(dcf_ctx *c)
+// The basin build's scratch is the largest buffer that contexts and batches keep, and both
+// can do without it: when the device is out of memory it is given back and the allocation
+// tried again (not while a build still has launches or copies on it to issue).  A batch
+// merges from then on; `optional` allocations, those of another such scratch, leave it its
+// own.
+static bool batch_give_back(dcf_ctx *c, dcf_batch *b);
+static void orphan_batch(dcf_batch *b);
+static bool give_back_forest(dcf_ctx *c, bool optional)
 {
-    if (!c || c->forest_busy || !c->scratch[FOREST_SLOT].p) return false;
+    if (!c) return false;
     cudaGetLastError();
-    cudaStreamSynchronize(c->stream);
-    cudaFree(c->scratch[FOREST_SLOT].p);
-    c->scratch[FOREST_SLOT] = DevBuf();
-    return true;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
+    if (!c->forest_busy && c->scratch[FOREST_SLOT].p) {
+        cudaStreamSynchronize(c->stream);
+        cudaFree(c->scratch[FOREST_SLOT].p);
+        c->scratch[FOREST_SLOT] = DevBuf();
+        return true;
+    }
+    if (optional) return false;
+    std::lock_guard<std::mutex> lk(c->trees_mu);
+    for (dcf_batch *b : c->batches)
+        if (batch_give_back(c, b)) return true;
+    return false;
 }
 template <typename T>
-static cudaError_t dmalloc(dcf_ctx *c, T **p, size_t bytes)
+static cudaError_t dmalloc(dcf_ctx *c, T **p, size_t bytes, bool optional = false)
 {
     if (alloc_refused(c)) return cudaErrorMemoryAllocation;
     cudaError_t e = device_full(c) ? cudaErrorMemoryAllocation : cudaMalloc((void **)p, bytes);
-    if (e == cudaErrorMemoryAllocation && give_back_forest(c)) e = cudaMalloc((void **)p, bytes);
+    while (e == cudaErrorMemoryAllocation && give_back_forest(c, optional)) e = cudaMalloc((void **)p, bytes);
     return e;
 }
 template <typename T>
@@ -224,7 +238,7 @@ static cudaError_t dmalloc_async(dcf_ctx *c, T **p, size_t bytes, cudaStream_t s
 {
     if (alloc_refused(c)) return cudaErrorMemoryAllocation;
     cudaError_t e = device_full(c) ? cudaErrorMemoryAllocation : cudaMallocAsync((void **)p, bytes, s);
-    if (e == cudaErrorMemoryAllocation && give_back_forest(c)) e = cudaMallocAsync((void **)p, bytes, s);
+    while (e == cudaErrorMemoryAllocation && give_back_forest(c, false)) e = cudaMallocAsync((void **)p, bytes, s);
     return e;
 }
 
@@ -263,7 +277,7 @@ static dcf_status scratch(dcf_ctx *ctx, int slot, size_t bytes, void **out)
         if (b.p) CU(cudaFree(b.p));
         b.p = nullptr;
         b.bytes = 0;
-        CU(dmalloc(ctx, &b.p, bytes));
+        CU(dmalloc(ctx, &b.p, bytes, slot == FOREST_SLOT));
         b.bytes = bytes;
     }
     *out = b.p;
@@ -391,6 +405,7 @@ dcf_status dcf_ctx_destroy(dcf_ctx *ctx)
         std::lock_guard<std::mutex> lk(ctx->trees_mu);
         for (dcf_tree *t : ctx->trees) orphan_tree(t);
         ctx->trees.clear();
+        for (dcf_batch *b : ctx->batches) orphan_batch(b);
     }
     if (ctx->stage.p) cudaFreeAsync(ctx->stage.p, ctx->stream);
     for (auto &b : ctx->scratch)
@@ -1478,7 +1493,10 @@ struct dcf_batch {
     unsigned rest_cap = 0;                   // graph runs: pointer-jumping capacity (0: not learned yet)
     size_t rest_bytes = 0;
     void *rest_mem = nullptr;
-    unsigned char *flag = nullptr;
+    unsigned char *flag = nullptr;           // flags, or the scratch of the direct rule along the chain order
+    size_t flag_bytes = 0;
+    bool chain_targets = false;              // which of the two the last run's targets are of
+    bool busy = false;                       // a run is using the basin scratch
     int *target = nullptr;
     float *filtered = nullptr;               // host-output staging
     double *spectra = nullptr;
@@ -1514,6 +1532,31 @@ static void batch_drop_graph(dcf_batch *b)
         if (g.graph) cudaGraphDestroy(g.graph);
     }
     b->graphs.clear();
+}
+
+static void orphan_batch(dcf_batch *b) { b->ctx = nullptr; }
+
+// The trees of the last run stay as they are; later runs merge.
+static bool batch_give_back(dcf_ctx *c, dcf_batch *b)
+{
+    if (b->busy || !b->forest_mem) return false;
+    cudaStreamSynchronize(c->stream);
+    batch_drop_graph(b);
+    cudaFree(b->forest_mem);
+    cudaFree(b->d_ftiles);
+    b->forest_mem = nullptr;
+    b->d_ftiles = nullptr;
+    b->forest = ForestWork();
+    b->chains = ChainOrder();
+    b->rest_cap = 0;  // counted chains; nodes are learned anew
+    return true;
+}
+
+// the node words of a batch that merges
+static dcf_status batch_ensure_node(dcf_ctx *ctx, dcf_batch *b)
+{
+    if (!b->forest_mem && !b->node) CU(dmalloc(ctx, &b->node, (size_t)b->N * 8));
+    return DCF_OK;
 }
 
 static TreeView batch_view(const dcf_batch *b)
@@ -1763,7 +1806,7 @@ static dcf_status batch_forest(dcf_ctx *ctx, dcf_batch *b)
     const size_t order_b = ((size_t)b->N * 4 + 255) / 256 * 256, work_b = bytes;
     bytes += order_b + (size_t)chain_blocks(b->N) * 4;
     cudaError_t e = dmalloc(ctx, &b->d_ftiles, tl.size() * sizeof(BatchTile));
-    if (e == cudaSuccess) e = dmalloc(ctx, &b->forest_mem, bytes);
+    if (e == cudaSuccess) e = dmalloc(ctx, &b->forest_mem, bytes, true);
     if (e == cudaErrorMemoryAllocation && ctx->fail_alloc < 0) {
         cudaGetLastError();
         return DCF_OK;
@@ -1887,6 +1930,10 @@ dcf_status dcf_batch_create(dcf_ctx *ctx, int count, const uint32_t *widths, con
     if ((st = batch_set_tiles(ctx, b, 64, 64, 0, 1)) != DCF_OK) goto fail;
     if (takes_basin_build(ctx, N) && (st = batch_forest(ctx, b)) != DCF_OK) goto fail;
     if (!b->forest_mem) BTRY(dmalloc(ctx, &b->node, (size_t)N * 8));
+    {
+        std::lock_guard<std::mutex> lk(ctx->trees_mu);
+        ctx->batches.insert(b);
+    }
     *out = b;
     return DCF_OK;
 fail:
@@ -1898,7 +1945,13 @@ fail:
 dcf_status dcf_batch_destroy(dcf_batch *b)
 {
     if (!b) return DCF_ERR_INVALID;
-    if (b->ctx) cudaStreamSynchronize(b->ctx->stream);
+    if (b->ctx) {
+        {
+            std::lock_guard<std::mutex> lk(b->ctx->trees_mu);
+            b->ctx->batches.erase(b);
+        }
+        cudaStreamSynchronize(b->ctx->stream);
+    }
     batch_drop_graph(b);
     void *bufs[] = {b->d_imgs, b->d_offs, b->d_tiles, b->d_misc, b->pixels, b->gval, b->node, b->parent, b->isroot,
                     b->nodes, b->attr_mem, b->rest_mem, b->flag, b->target, b->filtered, b->spectra, b->lvec, b->adj_acc,
@@ -1916,7 +1969,7 @@ dcf_status dcf_batch_info(const dcf_batch *b, uint64_t *total_pixels, uint64_t *
     if (total_pixels) *total_pixels = (uint64_t)b->N;
     if (num_nodes) {
         unsigned long long n = 0;
-        if (b->valid) {
+        if (b->valid && b->ctx) {
             cudaStreamSynchronize(b->ctx->stream);
             cudaMemcpy(&n, b->d_nodes, sizeof(n), cudaMemcpyDeviceToHost);
         }
@@ -1963,6 +2016,10 @@ dcf_status dcf_batch_autotune(dcf_ctx *ctx, dcf_batch *b, const void *pixels, in
     ActiveScope active_scope_(ctx);
     if (!ctx || !b || !pixels) return DCF_ERR_INVALID;
     if (repeats < 1) repeats = 1;
+    {
+        const dcf_status st = batch_ensure_node(ctx, b);
+        if (st != DCF_OK) return st;
+    }
     static const size_t esize[4] = {1, 2, 4, 4};
     const void *px = pixels;
     if (!on_device) {
@@ -2083,11 +2140,9 @@ dcf_status dcf_batch_autotune(dcf_ctx *ctx, dcf_batch *b, const void *pixels, in
     return finish(st, best_t);
 }
 
-dcf_status dcf_batch_run(dcf_ctx *ctx, dcf_batch *b, const void *pixels, int pixels_on_device, const dcf_op_set *ops,
-                         float *filtered, double *spectra, int outputs_on_device)
+static dcf_status batch_run(dcf_ctx *ctx, dcf_batch *b, const void *pixels, int pixels_on_device,
+                            const dcf_op_set *ops, float *filtered, double *spectra, int outputs_on_device)
 {
-    ActiveScope active_scope_(ctx);
-    if (!ctx || !b || !pixels || !ops) return DCF_ERR_INVALID;
     dcf_op_set o = *ops;
     if (o.filter_attr >= DCF_NUM_ATTRIBUTES || (o.filter_attr > 0 && ATTR_GROUP[o.filter_attr] != b->group))
         return set_err(ctx, DCF_ERR_INVALID, "filter attribute %d is not in the batch's group", o.filter_attr);
@@ -2102,10 +2157,19 @@ dcf_status dcf_batch_run(dcf_ctx *ctx, dcf_batch *b, const void *pixels, int pix
     const size_t N = (size_t)b->N;
     cudaStream_t s = ctx->stream;
     // buffers the requested operations need (allocated once)
-    if (o.filter_attr >= 0 && !b->flag) {
-        // flags, or the scratch of the direct rule along the chain order
-        CU(dmalloc(ctx, &b->flag, batch_chain_filter(b) ? chain_filter_bytes(b->N, batch_view(b).chain_cap) : N));
-        CU(dmalloc(ctx, &b->target, N * 4));
+    if ((st = batch_ensure_node(ctx, b)) != DCF_OK) return st;
+    if (o.filter_attr >= 0) {
+        const size_t need = batch_chain_filter(b) ? chain_filter_bytes(b->N, batch_view(b).chain_cap) : N;
+        if (b->flag_bytes < need) {
+            batch_drop_graph(b);
+            if (b->flag) CU(cudaFree(b->flag));
+            b->flag = nullptr;
+            b->flag_bytes = 0;
+            CU(dmalloc(ctx, &b->flag, need));
+            b->flag_bytes = need;
+        }
+        if (!b->target) CU(dmalloc(ctx, &b->target, N * 4));
+        b->chain_targets = batch_chain_filter(b);
     }
     if (filtered && !outputs_on_device && !b->filtered) CU(dmalloc(ctx, &b->filtered, N * 4));
     const size_t nspec = o.spec_attr1 >= 0 ? (size_t)b->count * o.n1 * o.n2 : 0;
@@ -2227,6 +2291,26 @@ dcf_status dcf_batch_run(dcf_ctx *ctx, dcf_batch *b, const void *pixels, int pix
     return DCF_OK;
 }
 
+dcf_status dcf_batch_run(dcf_ctx *ctx, dcf_batch *b, const void *pixels, int pixels_on_device, const dcf_op_set *ops,
+                         float *filtered, double *spectra, int outputs_on_device)
+{
+    ActiveScope active_scope_(ctx);
+    if (!ctx || !b || !pixels || !ops) return DCF_ERR_INVALID;
+    auto run = [&]() {
+        b->busy = true;
+        const dcf_status st = batch_run(ctx, b, pixels, pixels_on_device, ops, filtered, spectra, outputs_on_device);
+        b->busy = false;
+        return st;
+    };
+    dcf_status st = run();
+    // without room for its buffers beside the basin scratch a batch merges
+    if (st == DCF_ERR_NOMEM && ctx->fail_alloc < 0 && batch_give_back(ctx, b)) {
+        cudaGetLastError();
+        st = run();
+    }
+    return st;
+}
+
 __global__ void k_batch_local_parent(long long n, const int *__restrict__ parent, const long long *__restrict__ offs,
                                      int count, long long *out)
 {
@@ -2323,7 +2407,7 @@ dcf_status dcf_batch_adjoint(dcf_ctx *ctx, dcf_batch *b, const float *grad_filte
     CU(cudaMemsetAsync(b->adj_acc, 0, N * 8, s));
     AdjointArgs j;
     j.target = grad_filtered ? b->target : nullptr;
-    if (batch_chain_filter(b) && b->flag) j.base = chain_base(b->flag, b->N);
+    if (b->chain_targets) j.base = chain_base(b->flag, b->N);
     j.v = v;
     j.w = grad_spectra ? w : nullptr;
     j.a1 = o.spec_attr1;

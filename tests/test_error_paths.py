@@ -174,6 +174,46 @@ def test_builds_on_a_full_device(monkeypatch):
     assert recovered >= 10
 
 
+def test_batches_on_a_full_device(monkeypatch):
+    """The same for batches: whichever allocation finds the device full, runs, graphs and
+    gradients of the batch come out as they do with room, from basins or merged."""
+    _torch()
+    monkeypatch.delenv("DCF_FAIL_ALLOC", raising=False)
+    shapes = [(40, 50), (70, 33), (128, 96)]
+    rng = np.random.default_rng(2)
+    cuts = [rng.standard_normal(s).astype(np.float32) for s in shapes]
+    n = sum(h * w for h, w in shapes)
+    lv1, lv2 = dcf.lvec_from_values([10, 1e3, 1e5]), dcf.lvec_from_values([4, 16, 64, 256])
+    v, w = rng.standard_normal(n).astype(np.float32), rng.standard_normal((len(shapes), lv2.size, lv1.size))
+
+    def calls(ctx):
+        b = ctx.batch(shapes, np.float32, connectivity=8, attribute=13)
+        pix, out = b.concat(cuts), []
+        for graph in (False, True, True):
+            out += list(b.run(pix, filter_attr=0, lam=10.0, spectrum=(13, lv1, 0, lv2), use_graph=graph))
+            out += [b.adjoint(v, w), b.parent()]
+        b.close()
+        return out
+
+    ref = dcf.Context(0)
+    want = calls(ref)
+    ref.close()
+    for k in range(64):
+        ctx = knob_ctx(monkeypatch, "DCF_SHORT_ALLOC", k)
+        try:
+            got = calls(ctx)
+        except dcf.DcfError as e:  # before there is any scratch to give back
+            assert e.status == NOMEM and k < 20, (k, str(e))
+            ctx.close()
+            continue
+        for i, (g, x) in enumerate(zip(got, want)):
+            if g.dtype == np.float64 or i % 4 == 2:  # sums in another order
+                np.testing.assert_allclose(g, x, rtol=1e-6 if i % 4 == 2 else 1e-12, atol=1e-6 * np.abs(x).max())
+            else:
+                assert np.array_equal(g, x), (k, i)
+        ctx.close()
+
+
 def test_builds_and_attribute_passes_are_refused_under_capture():
     torch = _torch()
     stream = torch.cuda.Stream()

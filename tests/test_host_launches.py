@@ -224,3 +224,53 @@ def test_min_rule_without_room_for_the_chains_scratch(run):
         """)
     assert said == ["0"]
     assert any("k_jump_last" in r[1] for r in rows)
+
+
+BATCH = """
+shapes = [(1000, 1400), (700, 900)]
+n = sum(h * w for h, w in shapes)
+pix = np.zeros(n, np.float32)
+lv = np.float32([0, 1, 2])
+ctx = dcf.Context(0)
+b = ctx.batch(shapes, np.float32, connectivity=8, attribute=13)
+ops = dict(filter_attr=0, lam=3.0, spectrum=(13, lv, 0, lv))
+"""
+
+
+def test_batch_gives_its_scratch_back_for_its_own_buffers(run):
+    """Room for less than a run's buffers beside the basin scratch: the batch merges."""
+    said, rows = run(BATCH + """
+memory.value = in_use.value + n
+for graph in (False, True, True):
+    print(status(lambda: b.run(pix, use_graph=graph, **ops)))
+    print(status(lambda: b.adjoint(np.ones(n, np.float32), np.ones((2, 3, 3)))))
+print(status(lambda: b.autotune(pix, repeats=1)))
+""")
+    assert said == ["0"] * 7
+    assert not any("k_basins" in r[1] for r in rows) and any("k_batch_tile_build" in r[1] for r in rows)
+
+
+def test_batch_gives_its_scratch_back_after_a_run(run):
+    """The gradient, the parents or a tree that finds no room takes an idle batch's scratch;
+    another batch's own scratch does not."""
+    for call in ("b.adjoint(np.ones(n, np.float32), np.ones((2, 3, 3)))", "b.parent()", "b.node_attribute(13)",
+                 "ctx.build(np.zeros((1000, 800), np.float32), connectivity=8, tree_type='max', attribute=13)"):
+        said, rows = run(BATCH + f"""
+print(status(lambda: b.run(pix, use_graph=False, **ops)))
+memory.value = in_use.value + n
+print(status(lambda: {call}))
+print(ctx.launches)
+print(status(lambda: b.run(pix, use_graph=False, **ops)))
+""")
+        assert [said[i] for i in (0, 1, 3)] == ["0"] * 3, call
+        later = "".join(r[1] for r in rows[int(said[2]):])
+        assert "k_batch_tile_build" in later and "k_basins" not in later, call
+    said, rows = run(BATCH + """
+memory.value = in_use.value + 120 * n  # room for another batch without the scratch
+c = ctx.batch(shapes, np.float32, connectivity=8, attribute=13)
+at = ctx.launches
+print(status(lambda: c.run(pix, use_graph=False)), status(lambda: b.run(pix, use_graph=False)))
+""")
+    names = [r[1] for r in rows]
+    assert said == ["0", "0"]
+    assert sum("k_batch_tile_build" in k for k in names) == 1 and sum("k_basins" in k for k in names) == 1
