@@ -63,8 +63,11 @@ struct dcf_ctx {
     // short_alloc (DCF_SHORT_ALLOC = k): the k-th allocation finds the device full
     // instead, as it is for a user whose other buffers fill it: the library then gives
     // back what it keeps and tries again, or does without.
+    // edge_cap (DCF_EDGE_CAP): saddle edges a 3-D image may have in the basin build, below
+    // what its scratch holds; more send the image to the merging build.
     long long fail_alloc = -1;
     long long short_alloc = -1;
+    long long edge_cap = 0;
     long long allocs = 0;
     cudaEvent_t input_read = nullptr; // the last build has read its input
     bool forest_busy = false;         // a build is being launched on scratch[FOREST_SLOT]
@@ -367,6 +370,7 @@ dcf_status dcf_ctx_create(int device, void *cuda_stream, dcf_ctx **out)
     }
     if (const char *e = getenv("DCF_FAIL_ALLOC")) ctx->fail_alloc = atoll(e);
     if (const char *e = getenv("DCF_SHORT_ALLOC")) ctx->short_alloc = atoll(e);
+    if (const char *e = getenv("DCF_EDGE_CAP")) ctx->edge_cap = atoll(e);
     if (const char *e = getenv("DCF_UP_STEPS")) {
         int v = atoi(e);
         if (v >= 0 && v < (1 << 20)) ctx->up_steps = v;
@@ -816,6 +820,7 @@ static dcf_status tree_build(dcf_ctx *ctx, const dcf_image *img, int attr_idx, d
                 goto fail;
             }
             ba.forest = forest_carve(fm, conn, (long long)N, ba.basin_cap, nullptr);
+            if (D > 1 && ctx->edge_cap > 0) ba.forest.ecap = std::min(ba.forest.ecap, ctx->edge_cap);
             ctx->forest_busy = true;
             const cudaError_t e = alloc_order(ctx, t, ba.forest, ba.basin_cap);
             *redo = e == cudaErrorMemoryAllocation && ctx->fail_alloc < 0;

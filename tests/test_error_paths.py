@@ -214,6 +214,30 @@ def test_batches_on_a_full_device(monkeypatch):
         ctx.close()
 
 
+@pytest.mark.parametrize("conn", [6, 26])
+def test_volumes_with_more_saddles_than_the_scratch_holds(monkeypatch, conn):
+    """No volume is known to have more than two saddle edges a pixel, which is what the
+    scratch holds; a lower bound by knob shows that such a one would be merged, and that the
+    context then takes what fits as before."""
+    _torch()
+    vol, few = image(shape=(20, 30, 25)), np.zeros((20, 30, 25), np.uint16)
+    few[3, 4, 5] = 9
+    port = oracle.Port()
+    for cap in (1, 60, 1500):
+        ctx = knob_ctx(monkeypatch, "DCF_EDGE_CAP", cap)
+        ctx.set_profiling()
+        for x, merged in ((vol, True), (few, False), (vol, True)):
+            before = ctx.profile().get("tile_build", (0, 0))[1]
+            t = ctx.build(x, connectivity=conn, tree_type="max", attribute=0)
+            port.load(x.astype(np.float32), conn, "max")
+            port.prepare(0)
+            assert np.array_equal(t.parent(), port.parent())
+            assert np.array_equal(t.filter(0, 50.0), port.filter(0, 50.0, 0))
+            assert (ctx.profile().get("tile_build", (0, 0))[1] > before) == merged, (cap, merged)
+            t.close()
+        ctx.close()
+
+
 def test_builds_and_attribute_passes_are_refused_under_capture():
     torch = _torch()
     stream = torch.cuda.Stream()
