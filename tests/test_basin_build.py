@@ -249,3 +249,24 @@ def test_more_rows_and_slices_than_a_grid_has(builds):
     two = row[:2 * (m // 2)]
     got, flat = parents(two.reshape(2, -1, 1), 6), parents(two.reshape(2, -1), 4)
     assert np.array_equal(got, flat)
+
+
+@pytest.mark.gpu
+def test_large_batches_same_as_single_images(builds):
+    """A batch of 2^25 pixels and more writes its parents by way of buckets, over cutouts that
+    share buckets and blocks; each of its cutouts alone does not."""
+    shapes = [(3000, 3333), (2777, 4100), (1, 5000), (4096, 2500), (333, 444), (1501, 1999)]
+    assert sum(h * w for h, w in shapes) >= 1 << 25 > max(h * w for h, w in shapes)
+    rng = np.random.default_rng(12)
+    cuts = [(rng.integers(0, 60, s) * 3 + np.arange(s[1]) % 67).astype(np.uint16) for s in shapes]
+    b = builds[0].batch(shapes, np.uint16, connectivity=8, attribute=0)
+    lv = dcf.lvec_from_values([2, 8, 32, 128, 1024])
+    f, spec = b.run(b.concat(cuts), filter_attr=0, lam=9.0, spectrum=(0, lv, 0, lv), use_graph=False)
+    par, f = b.split(b.parent()), b.split(f)
+    for i, c in enumerate(cuts):
+        t = builds[0].build(c, connectivity=8, tree_type="max", attribute=0)
+        assert np.array_equal(par[i].ravel(), t.parent()), i
+        assert np.array_equal(f[i], t.filter(0, 9.0)), i
+        assert np.array_equal(spec[i], t.pattern_spectrum2d(0, lv, 0, lv)), i  # integers below 2^53
+        t.close()
+    b.close()
