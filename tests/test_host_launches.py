@@ -163,7 +163,7 @@ def test_tall_images_are_built(run, shape, conn):
 
 
 def test_merging_build_refuses_what_its_launch_cannot_hold(run):
-    """The merging build's tiles are a 3-D grid: taller images end at its tile kernel."""
+    """The merging build's tiles are a plain 3-D grid: taller images end at its tile kernel."""
     said, rows = run("""
         ctx = dcf.Context(0)
         print(status(lambda: ctx.build(np.zeros((2_097_121, 1), np.uint8), connectivity=4, tree_type="max", attribute=0)))
