@@ -31,9 +31,11 @@
 //               a run of equal keys take its first, lowest pixel, that one the run below
 //               it or, at the chain's end, the node of s(c).
 //
-// What bounds it: memory traffic of a fixed number of passes (24 bytes a pixel and sort
-// pass, parents written out of order), and for images below about a megapixel the latency
-// of some 20 kernels and of the grid barriers in k_saddles.  Build alone (without node list
+// What bounds it, on images beyond a few megapixels: in k_basins, k_chain and the sort's
+// first pass instructions (4096^2 u16: 64 to 67% of the issue slots with half the warps
+// resident, DRAM at 8 to 35%), in the other passes the latency of shared memory, gathers
+// and stores out of order (DRAM at 17 to 48%).  Below about a megapixel the latency of some
+// 20 kernels and of the grid barriers in k_saddles.  Build alone (without node list
 // and attributes) on GB300 against the merging build:
 //   1447 x 1083 f32, 8-connected                     0.32 ms   200 ms
 //   128 x 120 x 112 f32, 6-connected                 0.25 ms   141 ms
@@ -597,8 +599,9 @@ __device__ __forceinline__ int sort_passes(int key_bits, const unsigned *ctr)
 
 // Sort keys (chain, key), and how often every digit of every sort pass occurs.  The way to a
 // pixel's chain is a chain of dependent loads, so a thread takes four pixels at a time, a step
-// of each in turn; what bounds it is the deepest of a warp's pixels, and one large block an SM
-// does as well as more and flushes its counts once (with copies of the counts by lane the
+// of each in turn, as many as the deepest of a warp's pixels needs.  Instructions take 67% of
+// the issue slots (4096^2 u16, half the warps, DRAM at 20%), and one large block an SM does as
+// well as more and flushes its counts once (with copies of the counts by lane the
 // same).  One pixel at a time and eight blocks of 256 an SM took 26 us at 1447 x 1083 f32 and
 // 19 at 1024^2 u8; now 23 and 14 (four at a time with those blocks: 22 and 18; 8190 x 8211 u16
 // 637, now 583; eight at a time 28 and 14, 608).

@@ -29,7 +29,7 @@ namespace dcf {
 constexpr int STATS_THREADS = 256;
 // Bound by memory on large images (16384^2 u16: 0.09 ms, 88% of the copy rate, from
 // 0.17), by latency on small ones: a few blocks per SM, 16-byte loads, and one set of
-// atomics per block instead of per warp (1024^2 u8: 4 us, from 48, which were 65 536
+// atomics per block instead of per warp (1024^2 u8: 8 us, from 48, which were 65 536
 // atomics on two words).
 template <typename T>
 __global__ void __launch_bounds__(STATS_THREADS) k_stats(const T *__restrict__ img, long long n, unsigned *kmin,
