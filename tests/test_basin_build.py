@@ -270,3 +270,29 @@ def test_large_batches_same_as_single_images(builds):
         assert np.array_equal(spec[i], t.pattern_spectrum2d(0, lv, 0, lv)), i  # integers below 2^53
         t.close()
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+@pytest.mark.parametrize("shape", [(2, 1, 1), (2, 32, 32), (2, 32, 33), (9, 17, 17), (40, 50, 60), (1, 77), (64, 65), (300, 411)])
+def test_filters_on_costly_attributes_same_as_on_merged_trees(builds, shape, dtype):
+    """The sweeps along the chain order list a block's level roots before they evaluate an
+    attribute other than the area, and eigenvalues are evaluated node by node before them
+    (volumes, and images with pixels that are not unit squares): at the edges of a block of
+    2048 positions, for every way and rule, same images as the general path."""
+    volume = len(shape) == 3
+    for kind in ("noise", "few", "flat"):
+        img = image(shape, kind, dtype, 23)
+        img = np.where(np.isfinite(img.astype(np.float64)), img, 0).astype(dtype)
+        for pixdim in ((1.0, 1.0, 1.0), (1.0, 2.0, 1.0)):
+            t = [c.build(img, connectivity=6 if volume else 4, tree_type="max", attribute=14, pixdim=pixdim) for c in builds]
+            for attr in (14, 16, 13) + ((15,) if volume else ()):
+                lams = np.nanquantile(t[1].node_attribute(attr), [0.3, 0.9])
+                for lam in (float(lams[0]), float(lams[1]), 1e12):
+                    for rule in ("direct", "min", "subtractive"):
+                        if dtype == np.float32 and rule == "subtractive":
+                            continue  # the float recurrence is the same code on both trees
+                        got, want = (x.filter(attr, lam, rule) for x in t)
+                        assert np.array_equal(got, want), (kind, pixdim, attr, lam, rule)
+            for x in t:
+                x.close()
