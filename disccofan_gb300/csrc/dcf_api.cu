@@ -170,7 +170,7 @@ struct dcf_tree {
     int *parent = nullptr;
     unsigned char *isroot = nullptr;
     int *nodes = nullptr;                    // level roots in ascending order (node_list_bytes)
-    unsigned *stats = nullptr;               // kmin, kmax, nans of the input
+    unsigned *stats = nullptr;               // kmin, kmax, nans of the input; chains; node count (64 bits)
     unsigned long long *num_nodes = nullptr;
     AttrBufs attr;
     int attr_idx = -1;
@@ -178,6 +178,7 @@ struct dcf_tree {
     // trees of the basin build: the chain order (n > 0) and its memory
     ChainOrder chains;
     unsigned chain_cap = 0;                  // entries of the chain tables
+    unsigned long long known_nodes = ~0ull;  // the node count, where the build read it back
     void *order_mem = nullptr, *table_mem = nullptr;
 };
 
@@ -650,7 +651,7 @@ static cudaError_t alloc_order(dcf_ctx *ctx, dcf_tree *t, ForestWork &w, long lo
     const bool bound = t->g.D == 1 && (size_t)t->chain_cap * 12 <= CHAIN_TABLE_BOUND;
     const size_t order_b = up((size_t)t->g.N * 4), first_b = up((size_t)chain_blocks(t->g.N) * 4),
                  row = bound ? up((size_t)t->chain_cap * 4) : 0;
-    cudaError_t e = dmalloc_async(ctx, &t->order_mem, order_b + first_b + 3 * row + 4, ctx->stream);
+    cudaError_t e = dmalloc_async(ctx, &t->order_mem, order_b + first_b + 3 * row, ctx->stream);
     if (e != cudaSuccess) return e;
     char *m = (char *)t->order_mem;
     t->chains.order = (int *)m;
@@ -661,7 +662,7 @@ static cudaError_t alloc_order(dcf_ctx *ctx, dcf_tree *t, ForestWork &w, long lo
         t->chains.up = w.up = (int *)(m + row);
         t->chains.kids = w.kids = (int *)(m + 2 * row);
     }
-    t->chains.nchains = (unsigned *)(m + 3 * row);
+    t->chains.nchains = t->stats + 3;
     return e;
 }
 
@@ -674,8 +675,8 @@ static dcf_status keep_chains(dcf_ctx *ctx, dcf_tree *t, const ForestWork &w, bo
         t->chains.n = t->g.N;
         return DCF_OK;
     }
-    unsigned err = 0, n = 0;
-    CU(cudaMemcpyAsync(&n, t->chains.nchains, sizeof(n), cudaMemcpyDeviceToHost, ctx->stream));
+    unsigned err = 0, n[3] = {0, 0, 0};  // chains, and the node count behind them
+    CU(cudaMemcpyAsync(n, t->chains.nchains, sizeof(n), cudaMemcpyDeviceToHost, ctx->stream));
     CU(cudaMemcpyAsync(&err, ctx->d_err, sizeof(err), cudaMemcpyDeviceToHost, ctx->stream));
     CU(cudaStreamSynchronize(ctx->stream));
     if (err & DEVERR_CAPACITY) {
@@ -685,7 +686,8 @@ static dcf_status keep_chains(dcf_ctx *ctx, dcf_tree *t, const ForestWork &w, bo
         *redo = true;
         return DCF_ERR_NOMEM;
     }
-    if (n < t->chain_cap) t->chain_cap = n;
+    t->known_nodes = n[1] | (unsigned long long)n[2] << 32;
+    if (n[0] < t->chain_cap) t->chain_cap = n[0];
     const size_t bytes = (size_t)t->chain_cap * 4, row = (bytes + 255) / 256 * 256;
     const cudaError_t e = dmalloc_async(ctx, &t->table_mem, 3 * row, ctx->stream);
     *redo = e == cudaErrorMemoryAllocation && ctx->fail_alloc < 0;
@@ -1123,12 +1125,27 @@ static long long depth_bound(const dcf_tree *t)
     return t->g.N;
 }
 
+// Whether the direct rule goes along the chain order, whose sweeps read every pixel's entry, or
+// by flags and halving, which touch the nodes alone but share the steps of long paths.  Paths of
+// u8 images are short (see direct_targets).  Where the build has read back how many nodes there
+// are (volumes, images from 1.4 to 2.8 Mpx on), few nodes go by halving too: at most one in
+// eight pixels, and at most 2^20 on paths of at most 65536 (u16), 2^16 on any.  u16 filter calls,
+// us, chain order and halving: flat 4096^2 120 and 61, 8192^2 400 and 164, mask 4096^2 143 and
+// 65, one ramp of 65536 levels 8192^2 453 and 204; noise 4096^2 (41% nodes) 310 and 393.  Beyond
+// 2^20 nodes halving still wins on shallow trees (8192^2, four levels: 743 and 436) but not on
+// deep ones (64 ramps of 65536 levels side by side: 840 and 7619).
+static bool chain_filter(const dcf_tree *t)
+{
+    if (!t->chains.n || t->dtype == U8) return false;
+    return t->known_nodes > (unsigned long long)std::min(t->g.N / 8, t->dtype == U16 ? 1ll << 20 : 1ll << 16);
+}
+
 // flags (or, for the direct rule of a tree with a chain order, its sweeps' scratch) and
 // targets
 static dcf_status direct_scratch(dcf_ctx *ctx, dcf_tree *t, int rule, FilterWork &w)
 {
     const size_t N = (size_t)t->g.N;
-    bool chain = rule == 0 && t->chains.n && t->dtype != U8;  // short paths: see direct_targets
+    bool chain = rule == 0 && chain_filter(t);
     void *p;
     dcf_status st;
     st = scratch(ctx, 1, chain ? chain_filter_bytes(t->g.N, t->chain_cap) : N, &p);

@@ -296,3 +296,20 @@ def test_filters_on_costly_attributes_same_as_on_merged_trees(builds, shape, dty
                         assert np.array_equal(got, want), (kind, pixdim, attr, lam, rule)
             for x in t:
                 x.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,flat", [(np.float32, 15), (np.float32, 100), (np.uint16, 60), (np.uint32, 40), (np.uint32, 60)])
+def test_direct_rule_of_one_long_path(builds, dtype, flat):
+    """A raster ramp is one path of N / flat nodes with areas N - k * flat: the direct rule goes
+    by nodes where these are few and along the chain order where they are more than 2^16."""
+    shape = (1800, 1901)
+    n = shape[0] * shape[1]
+    img = (np.arange(n) // flat).reshape(shape).astype(dtype)
+    t = builds[0].build(img, connectivity=4, tree_type="max", attribute=0)
+    assert t.info()["nodes"] == -(-n // flat)
+    for lam in (1, flat + 1, 5 * flat, 70_001, n // 2, n, n + 1):
+        kept = (n - lam) // flat if lam <= n else -1  # the highest surviving level
+        want = np.minimum(img, kept) if kept >= 0 else np.zeros(shape)
+        assert np.array_equal(t.filter(0, float(lam)), want.astype(np.float32)), lam
+    t.close()
