@@ -313,3 +313,40 @@ def test_direct_rule_of_one_long_path(builds, dtype, flat):
         want = np.minimum(img, kept) if kept >= 0 else np.zeros(shape)
         assert np.array_equal(t.filter(0, float(lam)), want.astype(np.float32)), lam
     t.close()
+
+
+@pytest.mark.gpu
+def test_many_contexts_at_once():
+    """Eight threads build on contexts of their own: the component rounds are a cooperative
+    kernel each, whose blocks wait for one another while the others' kernels run."""
+    import threading
+
+    imgs = [image((700 + 37 * k, 1500), "noise", np.float32 if k % 2 else np.uint16, 30 + k) for k in range(8)]
+    imgs = [np.where(np.isfinite(i.astype(np.float64)), i, 0).astype(i.dtype) for i in imgs]
+    ctx = dcf.Context(0)
+    want = []
+    for img in imgs:
+        t = ctx.build(img, connectivity=8, tree_type="max", attribute=0)
+        want.append((t.parent(), t.filter(0, 30.0)))
+        t.close()
+    ctx.close()
+    bad = []
+
+    def work(k):
+        try:
+            c = dcf.Context(0)
+            for r in range(12):
+                t = c.build(imgs[k], connectivity=8, tree_type="max", attribute=0)
+                if not np.array_equal(t.filter(0, 30.0), want[k][1]) or (r % 4 == 0 and not np.array_equal(t.parent(), want[k][0])):
+                    bad.append((k, r))
+                t.close()
+            c.close()
+        except Exception as e:  # reported below, in the test's own thread
+            bad.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
